@@ -147,7 +147,7 @@ cudaError_t launch_batch(const FusedArgs* d_reqs, const BatchTile* d_tiles, cons
                          uint32_t* d_counter, int grid, cudaStream_t st);
 
 // lanes-per-frame kernels: N/64 lanes per frame, the FFT in registers
-// (power at windows 2^6 and 2^7, half-complex at 2^6)
+// (power at windows 2^6 .. 2^8, half-complex at 2^6)
 bool tpf_has(int exp, int outk);
 int tpf_frames_per_cta(int exp);
 int tpf_occupancy(int exp, int outk);

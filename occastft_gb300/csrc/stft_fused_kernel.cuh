@@ -116,14 +116,14 @@ __device__ __forceinline__ void power_pair(float2 xa, float2 xb, float& pa, floa
 // 1e8 samples, power_of against this, overlap 0.5 / 0.75 / dense layout:
 // 2^7 207.3 / 393 / 213 -> 205.3 / 381.5 / 204 us, 2^9 212.8 / 400 / 192.7 -> 208.5 / 388 / 182.8,
 // 2^10 206.4 / 395 / 194 -> 199.6 / 380 / 181.5, 2^11 230.7 / 451 / 214.5 -> 223.5 / 439 / 204.3.
-template <int OUTK, bool FIX>
+template <int OUTK, bool FIX, bool SHORT = OUTK == OUT_POWER>
 struct BinPower {
     float lowest = 3.0e38f;
     // returns the value; store: whether this pass writes it
     __device__ __forceinline__ float of(float2 x, bool& store)
     {
         store = true;
-        if constexpr (OUTK != OUT_POWER) {
+        if constexpr (!SHORT) {
             return power_of<OUTK>(x);
         } else {
             const float q = fmaf(x.x, x.x, x.y * x.y);
@@ -136,7 +136,7 @@ struct BinPower {
             }
         }
     }
-    __device__ __forceinline__ bool again() const { return OUTK == OUT_POWER && lowest < kMinNormal; }
+    __device__ __forceinline__ bool again() const { return SHORT && lowest < kMinNormal; }
 };
 __device__ __forceinline__ void stcs_if(bool store, float* p, float v)
 {
@@ -164,9 +164,9 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc)
 // F rows of N samples, `hop` apart at src, to rows RS floats apart in shared
 // memory, by one warp with no bounds (the caller checked the span): 8- or
 // 4-byte copies for frames that do not start on 16 bytes, a fixed column per
-// lane.  (With a division and bounds per copy, window 2^7 at an odd frame
-// advance took 590 us for 1e8 samples at overlap 0.3, 2.5 times the one-frame
-// kernel; now 189, against 219 for the best other kernel.)
+// lane.  (With a division and bounds per copy, windows 2^7 and 2^8 at an odd
+// frame advance took 590 us for 1e8 samples at overlap 0.3, 2.5 times the
+// one-frame kernel; now 192 and 209, against 244 and 227 for the best other kernel.)
 template <int N, int RS, int F>
 __device__ __forceinline__ void cp_async_rows(float* dst, const float* src, uint64_t hop, int lane, int cs)
 {

@@ -20,15 +20,15 @@ namespace ocs {
 // ------------------------------------------------------------ plan
 // Windows 2^8 (16 values per thread), 2^9 and 2^10 (32): a pair is one exchange
 // inside a warp, and 16 or 32 lanes store 64 or 128 bytes of a row at a time.
-// 1e8 samples at 2^8, power, overlap 0.5 / 0.75 / 0.3, the lanes-per-frame
-// kernel (four lanes, each reading its whole frame from shared memory) against
-// this: 240 / 459 / 204 -> 204 / 367 / 162 us; with 32 values and 8 lanes here
-// 296 / 548 / 223.  At 2^7 the lanes-per-frame kernel stays (205 us against 290
-// here with 16 values and 276 with 8, which take a second exchange), and at 2^6
-// (204; the pair plan is for outputs that do not start on 16 bytes, which that
-// kernel cannot write: 440 against 705 us for the one-frame kernel); at 2^11
-// the one-frame kernel is faster (one exchange; 241 against 330 us), above it
-// the mirror-group kernel.
+// 2^8 runs it only when asked to (OCS_KERNEL=pair), because two frames in one
+// FFT round relative to the louder of the two: 1e8 samples, power, overlap 0.5 /
+// 0.75 / 0.3, the lanes-per-frame kernel 240 / 459 / 204 us, this 204 / 367 /
+// 162; with 32 values and 8 lanes here 296 / 548 / 223.  At 2^7 the
+// lanes-per-frame kernel stays (205 us against 290 here with 16 values and 276
+// with 8, which take a second exchange), and at 2^6 (204; the pair plan is for
+// outputs that do not start on 16 bytes, which that kernel cannot write: 440
+// against 705 us for the one-frame kernel); at 2^11 the one-frame kernel is
+// faster (one exchange; 241 against 330 us), above it the mirror-group kernel.
 __host__ __device__ constexpr int pair_R(int pid) { return pid <= 8 ? 16 : 32; }
 
 __host__ __device__ constexpr FusedCfg pair_cfg(int pid)

@@ -1,4 +1,4 @@
-// Thread-per-frame STFT for windows 2^6 and 2^7 (sm_103a).
+// Thread-per-frame STFT for windows 2^6 .. 2^8 (sm_103a).
 //
 // At N = 64 the cooperative kernels spend most of their instructions on
 // moving data between the threads that share a frame (shuffles, exchange
@@ -17,19 +17,18 @@
 // Outputs: power (|X| or the Serial runner's sqrt(2)|Re X|) in the reference
 // layout or the dense layout; at N = 64 also half-complex (tpf_half_out).
 //
-// Window 2^7 uses L = 2 lanes per frame (stft_tpfl_kernel): the packed M-point
-// complex FFT (M = N / 2 = 64) starts with one radix-2 decimation-in-frequency
-// step that both lanes form on their own from the whole row, keeping only their
-// output q:
-//   u_q[n] = (z[n] + (-1)^q z[n + 32]) W_M^{n q},  n < 32,
-// and a 32-point DFT of u_q in registers gives Z[2k + q].  The untangle pairs
-// Z[k] with Z[M - k], both in the same lane.  Each lane then owns the bins
-// congruent to +-q mod 2 and writes them into the frame's row.  Power outputs
-// only.  (With four lanes per frame at 2^8 every lane reads four lanes' samples
-// from shared memory: 240 us for 1e8 samples against 204 in the paired kernel.)
-// It is the same pipeline as the fused kernels (Overlap_Common, Window_*,
-// DCRemove_Common, Stockham FFT, toPower / toHalfComplexFormat;
-// OKL/EXPCommon.okl:7-245, OKL/kernel.okl:178-218).
+// Windows 2^7 and 2^8 use L = N / 64 lanes per frame (stft_tpfl_kernel): the
+// packed M-point complex FFT (M = N / 2 = 32 L) starts with one radix-L
+// decimation-in-frequency step that every lane forms on its own from the whole
+// row, keeping only its output q:
+//   u_q[n] = (sum_p z[n + 32 p] W_L^{p q}) W_M^{n q},  n < 32,
+// and a 32-point DFT of u_q in registers gives Z[L k + q].  The untangle pairs
+// Z[k] with Z[M - k]; for L = 2 both sit in the same lane, for L = 4 lanes 1
+// and 3 swap their upper 16 slots with one shuffle each.  Each lane then owns
+// the bins congruent to +-q mod L and writes them into the frame's row.
+// Windows 2^7 and 2^8 produce power outputs.  It is the same pipeline as the
+// fused kernels (Overlap_Common, Window_*, DCRemove_Common, Stockham FFT,
+// toPower / toHalfComplexFormat; OKL/EXPCommon.okl:7-245, OKL/kernel.okl:178-218).
 #include "stft_tpfl_body.cuh"
 
 #include <cstring>
@@ -312,7 +311,7 @@ int occupancy_tpf_t()
     return blocks;
 }
 
-// ---------------------------------------------------------------- two lanes per frame
+// ---------------------------------------------------------------- L lanes per frame
 template <int EXP, int OUTK>
 __global__ void __launch_bounds__(TplCfg<EXP>::THREADS, 2) stft_tpfl_kernel(const FusedArgs a,
                                                                              const WinParam<1 << EXP> wp)
@@ -360,11 +359,12 @@ int occupancy_tpfl_t()
 bool tpf_has(int exp, int outk)
 {
     if (outk == OUT_HALF) return exp == 6;
-    return exp >= 6 && exp <= 7 && (outk == OUT_POWER || outk == OUT_POWER_SERIAL);
+    return exp >= 6 && exp <= 8 && (outk == OUT_POWER || outk == OUT_POWER_SERIAL);
 }
 int tpf_frames_per_cta(int exp)
 {
     if (exp == 7) return TplCfg<7>::THREADS / 32 * TplCfg<7>::F;
+    if (exp == 8) return TplCfg<8>::THREADS / 32 * TplCfg<8>::F;
     return kTpfThreads;
 }
 
@@ -379,6 +379,8 @@ cudaError_t launch_tpf(int exp, int outk, const FusedArgs& a, const float* host_
     case 6: return ser ? launch_tpf_t<6, OUT_POWER_SERIAL>(a, hw, grid, st) : launch_tpf_t<6, OUT_POWER>(a, hw, grid, st);
     case 7:
         return ser ? launch_tpfl_t<7, OUT_POWER_SERIAL>(a, hw, grid, st) : launch_tpfl_t<7, OUT_POWER>(a, hw, grid, st);
+    case 8:
+        return ser ? launch_tpfl_t<8, OUT_POWER_SERIAL>(a, hw, grid, st) : launch_tpfl_t<8, OUT_POWER>(a, hw, grid, st);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -391,6 +393,7 @@ int tpf_occupancy(int exp, int outk)
     switch (exp) {
     case 6: return ser ? occupancy_tpf_t<6, OUT_POWER_SERIAL>() : occupancy_tpf_t<6, OUT_POWER>();
     case 7: return ser ? occupancy_tpfl_t<7, OUT_POWER_SERIAL>() : occupancy_tpfl_t<7, OUT_POWER>();
+    case 8: return ser ? occupancy_tpfl_t<8, OUT_POWER_SERIAL>() : occupancy_tpfl_t<8, OUT_POWER>();
     default: return 0;
     }
 }

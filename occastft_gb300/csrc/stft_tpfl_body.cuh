@@ -1,26 +1,29 @@
-// Lanes-per-frame STFT body for window 2^7, power outputs (sm_103a): L = 2
-// lanes per frame, 16 frames per warp, the FFT in registers.  Shared by the
-// lanes-per-frame kernel (stft_tpf.cu) and the batch kernel's 2^7 power tiles
-// (stft_batch_kernel.cuh).
+// Lanes-per-frame STFT body for windows 2^7 and 2^8, power outputs (sm_103a):
+// L = N/64 lanes per frame, 32/L frames per warp, the FFT in registers.  Shared
+// by the lanes-per-frame kernel (stft_tpf.cu) and the batch kernel's power
+// tiles of those windows (stft_batch_kernel.cuh).
 //
-// The packed M-point complex FFT (M = N/2 = 64) begins with one radix-2
+// The packed M-point complex FFT (M = N/2 = 32 L) begins with one radix-L
 // decimation-in-frequency step: each lane forms its own output q of that step
-// from the whole row, u_q[n] = (z[n] + (-1)^q z[n + 32]) W_M^{nq}, n < 32, and
-// its 32-point DFT in registers is then Z[2k + q].  The untangle pairs Z[k] with
-// Z[M - k] (both in the same lane) and one untangle gives the powers of bins k,
-// N - k, M + k and M - k.  Frames come in by cp.async as padded shared rows and
-// leave through the same rows with coalesced stores.  Per frame it implements the reference's Overlap_Common ->
+// from the whole row, u_q[n] = (sum_p z[n + 32p] W_L^{pq}) W_M^{nq}, n < 32, and
+// its 32-point DFT in registers is then Z[Lk + q].  The untangle pairs Z[k] with
+// Z[M - k] (same lane for L = 2, lanes 1 and 3 swap for L = 4) and one untangle
+// gives the powers of bins k, N - k, M + k and M - k.  Frames come in by
+// cp.async as padded shared rows and leave through the same rows with
+// coalesced stores.  Per frame it implements the reference's Overlap_Common ->
 // Window_* -> DCRemove_Common -> FFT -> toPower (OKL/EXPCommon.okl:7-245,
 // OKL/kernel.okl:178-194).
 #pragma once
 #include "stft_fused_kernel.cuh"
+
+#include <type_traits>
 
 namespace ocs {
 
 // The window coefficients (scaled by 1/2) as float4s: a kernel parameter (every
 // lane reads the same coefficient at a compile-time offset, which the constant
 // cache serves without using the shared-memory / L1 pipe the kernels are bound
-// by; at most 512 bytes) or a copy in shared memory.
+// by; N <= 256: at most 1 KB) or a copy in shared memory.
 template <int N>
 struct WinParam {
     float4 v[N / 4];
@@ -60,13 +63,14 @@ constexpr TplTab<EXP> make_tpl_tab()
 
 namespace {  // one copy per translation unit that runs the body
 __constant__ TplTab<7> c_tpl7 = make_tpl_tab<7>();
+__constant__ TplTab<8> c_tpl8 = make_tpl_tab<8>();
 }  // namespace
 
 template <int EXP>
 __device__ __forceinline__ const TplTab<EXP>& tpl_tab()
 {
-    static_assert(EXP == 7, "window 2^7");
-    return c_tpl7;
+    if constexpr (EXP == 7) return c_tpl7;
+    else return c_tpl8;
 }
 
 template <int EXP>
@@ -105,9 +109,12 @@ __device__ __forceinline__ void tpfl_group(const FusedArgs& a, uint64_t g, float
     using C = TplCfg<EXP>;
     constexpr int N = C::N, M = C::M, L = C::L, F = C::F, RS = C::RS, ORS = C::ORS;
     static_assert(OUTK == OUT_POWER || OUTK == OUT_POWER_SERIAL, "power outputs only");
-    static_assert(L == 2, "window 2^7");
+    static_assert(L == 2 || L == 4, "windows 2^7 and 2^8");
     const int q = lane % L, jf = lane / L;  // lane q of the warp's frame jf
-    const float sq = q ? -1.0f : 1.0f;      // (-1)^q
+    // this lane's factors: W_4^q = (cr, ci) and (-1)^q = s2 (for L = 2, (-1)^q = cr)
+    const float cr = (L == 2) ? (q ? -1.0f : 1.0f) : (q == 0 ? 1.0f : q == 2 ? -1.0f : 0.0f);
+    const float ci = (L == 2) ? 0.0f : (q == 1 ? -1.0f : q == 3 ? 1.0f : 0.0f);
+    const float s2 = (q & 1) ? -1.0f : 1.0f;
 
     const int cs = a.cs;
     const int per_chunk = cs / 4;
@@ -192,8 +199,22 @@ __device__ __forceinline__ void tpfl_group(const FusedArgs& a, uint64_t g, float
         // The window products stay scalar: from the parameter bank they take
         // the coefficient as an operand, and packed ones made the batch
         // kernel spill.
-        v[2 * c] = fma2(bc2(sq), y0[1], y0[0]);  // z0 + (-1)^q z1
-        v[2 * c + 1] = fma2(bc2(sq), y1[1], y1[0]);
+        if constexpr (L == 2) {
+            // z0 + (-1)^q z1
+            v[2 * c] = fma2(bc2(cr), y0[1], y0[0]);
+            v[2 * c + 1] = fma2(bc2(cr), y1[1], y1[0]);
+        } else {
+            // (z0 + (-1)^q z2) + W_4^q (z1 + (-1)^q z3)
+            static_for<0, 2>([&](auto hc) {
+                constexpr int h = decltype(hc)::value;
+                const float2* y = h ? y1 : y0;
+                const float2 P = fma2(bc2(s2), y[2], y[0]);
+                const float2 Q = fma2(bc2(s2), y[3], y[1]);
+                // (cr Q.x + (-ci Q.y + P.x), cr Q.y + (ci Q.x + P.y))
+                const float2 inner = fma2(make_float2(-ci, ci), make_float2(Q.y, Q.x), P);
+                v[2 * c + h] = fma2(bc2(cr), Q, inner);
+            });
+        }
     }
     if (a.remove_dc) {
         // lane 0 of the frame summed every sample: its u_0 carries L means
@@ -212,6 +233,16 @@ __device__ __forceinline__ void tpfl_group(const FusedArgs& a, uint64_t g, float
     dft_inreg<32, 32, 0, 1>(v);  // Z[L k + q] in slot k
     __syncwarp();                 // every lane has read its row
 
+    float2 ex[L == 4 ? 16 : 1];
+    if constexpr (L == 4) {
+        // lanes q = 1 and 3 pair Z[4k + q] with Z[4(31 - k) + 4 - q]: the partner's slot 31 - k
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            ex[i].x = __shfl_xor_sync(0xffffffffu, v[16 + i].x, 2);
+            ex[i].y = __shfl_xor_sync(0xffffffffu, v[16 + i].y, 2);
+        }
+    }
+
     // ---------------- untangle, power, into the frame's row (bins = +-q mod L)
     float* orow = rows + jf * ORS;
     float* const Pp = orow + q;
@@ -222,7 +253,13 @@ __device__ __forceinline__ void tpfl_group(const FusedArgs& a, uint64_t g, float
             constexpr int kp = decltype(kc)::value;  // k = L kp + q
             if (kp == 16 && q != 0) return;          // k = M/2 belongs to q = 0
             const float2 A = v[kp];
-            const float2 B = q ? v[(63 - kp) % 32] : v[(32 - kp) % 32];
+            float2 B;
+            if constexpr (L == 2) {
+                B = q ? v[(63 - kp) % 32] : v[(32 - kp) % 32];
+            } else {
+                const float2 b0 = v[(32 - kp) % 32], b2 = v[(63 - kp) % 32], bx = ex[(31 - kp) % 16];
+                B = (q & 1) ? bx : (q ? b2 : b0);
+            }
             const float2 e = make_float2(A.x + B.x, A.y - B.y);
             const float2 od = make_float2(A.y + B.y, B.x - A.x);
             const float2 wo = cmul(od, s_tw2[kp * L + q]);
@@ -247,9 +284,11 @@ __device__ __forceinline__ void tpfl_group(const FusedArgs& a, uint64_t g, float
             }
         });
     };
-    BinPower<OUTK, false> power;
+    // the short root at 2^7 only (2^8: 239.5 -> 239.7 us, overlap 0.3 204 -> 206.6)
+    constexpr bool TWO_PASS = OUTK == OUT_POWER && L == 2;
+    BinPower<OUTK, false, TWO_PASS> power;
     bins(power);
-    if constexpr (OUTK == OUT_POWER) {
+    if constexpr (TWO_PASS) {
         if (power.again()) {
             BinPower<OUTK, true> fix;
             bins(fix);
@@ -260,7 +299,7 @@ __device__ __forceinline__ void tpfl_group(const FusedArgs& a, uint64_t g, float
     // ---------------- F rows -> HBM, coalesced
     const int nf = (a.frames - f0) < (uint64_t)F ? (int)(a.frames - f0) : F;
     if (!a.dense) {
-        using V = float2;
+        using V = typename std::conditional<L == 2, float2, float4>::type;
         constexpr int VPR = N / L;  // vectors per row, a multiple of 32
         V* dst = reinterpret_cast<V*>(a.out + f0 * (uint64_t)N);
         if (nf == F) {
