@@ -71,7 +71,7 @@ struct FusedArgs {
     uint64_t frames;       // frames to compute
     const float* win;      // window table scaled by 1/2 (N floats), never null
     const float2* tw;      // twiddle table of the plan
-    const float2* tw_pair; // batch kernels: the pair plan's or the mirror-group kernel's table (null: not used)
+    const float2* tw_pair; // batch kernels: the pair plan's table, from 2^12 the mirror-group kernel's (null: not used)
     float* out;            // output (or real plane)
     float* out_im;         // imaginary plane (planes mode)
     uint64_t ohalf;        // compat half-complex: number of complex outputs
@@ -103,17 +103,21 @@ int pair_twiddle_count(int pid);
 cudaError_t build_pair_twiddles(float2* tw, int pid, cudaStream_t st);
 
 // mirror-group kernel (stft_mirror_kernel.cuh), windows 2^12 .. 2^15: two
-// frames per transform up to 2^13, one above (a pair at 2^14 needs the threads
-// and shared memory of a frame at 2^15: 413 against 358 us for 1e8 samples,
-// power, overlap 0.5)
+// frames per transform for power up to 2^13 (batch tiles: up to 2^12, not the
+// Serial runner's), one otherwise.  A pair rounds relative to the louder of its
+// frames, so calls that held one frame per FFT before this kernel keep that; and
+// a pair at 2^14 needs the threads
+// and shared memory of a frame at 2^15 (413 against 358 us for 1e8 samples,
+// power, overlap 0.5).
 constexpr int kMirrorPlan = 64;  // flag of its plan ids (with log2 of its points)
-constexpr bool mirror_paired(int exp) { return exp <= 13; }
-constexpr int mirror_lp(int exp) { return mirror_paired(exp) ? exp : exp - 1; }  // log2 of its points
-constexpr int mirror_plan_id(int exp) { return kMirrorPlan + mirror_lp(exp); }   // for its twiddle table
+constexpr bool mirror_paired(int exp, int outk) { return exp <= 13 && outk != OUT_HALF; }
+constexpr bool batch_mirror_paired(int exp, int outk) { return exp == 12 && outk == OUT_POWER; }  // batch tiles
+constexpr int mirror_lp(int exp, bool pair) { return pair ? exp : exp - 1; }  // log2 of its points
+constexpr int mirror_plan_id(int exp, bool pair) { return kMirrorPlan + mirror_lp(exp, pair); }  // its twiddle table
 bool pairx2_has(int exp, int outk);
 cudaError_t launch_pairx2(int exp, int outk, const FusedArgs& a, int grid, cudaStream_t st);
 int pairx2_occupancy(int exp, int outk);
-int pairx2_per_cta(int exp);  // transforms per CTA
+int pairx2_per_cta(int exp);  // pairs of frames per CTA up to 2^13, frames above
 
 // uneven batch: persistent launches over device tile queues, one per window
 // size present (stft_batch_kernel.cuh)
@@ -122,13 +126,22 @@ struct BatchTile {
     uint32_t nframes;  // frames in this tile
     uint64_t f0;       // first frame
 };
-constexpr int kBatchMaxClasses = 8;  // windows 2^6 .. 2^13
-// the tiles of each window size, in the order of the tile list; class i's queue
+// The tiles of a batch fall into classes, one kernel each: the window size, and
+// at 2^12 the tiles of one frame per transform by themselves (with both forms in
+// one kernel the paired one spills, 73 -> 74.4 us for 64 requests).
+constexpr int kBatchMaxClasses = 9;  // windows 2^6 .. 2^13 and kBatchSingle12
+constexpr int kBatchSingle12 = 32 + 12;
+constexpr int batch_class(int exp, int outk)
+{
+    return exp == 12 && !batch_mirror_paired(exp, outk) ? kBatchSingle12 : exp;
+}
+constexpr int batch_class_exp(int cls) { return cls & 31; }
+// the tiles of each class, in the order of the tile list; class i's queue
 // counter is d_counter[i]
 struct BatchClasses {
     int count = 0;
     struct Class {
-        int exp;
+        int id;
         uint32_t begin, tiles;
     } cls[kBatchMaxClasses];
 };

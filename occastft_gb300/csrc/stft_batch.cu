@@ -9,8 +9,8 @@ size_t batch_smem_bytes() { return batch_smem(0); }
 bool batch_supports(int exp) { return exp >= kBatchMinExp && exp <= kBatchMaxExp; }
 // a tile is `groups` CTA-groups of frames (the host's autotuner picks the
 // count per batch mix; any count keeps tiles whole groups of every body)
-// -- at 2^13, where a CTA of the one-frame body holds one frame, groups of two
-// for the pairs
+// -- at 2^13, where a CTA of the one-frame kernel holds one frame, groups of two,
+// as the mirror-group body holds
 int batch_tile_frames(int exp, int groups) { return (exp == 13 ? 2 : fused_fpc(exp)) * groups; }
 
 int batch_occupancy()
@@ -20,15 +20,15 @@ int batch_occupancy()
     return std::min(std::min(lo, batch_occupancy_hi()), batch_occupancy_all());
 }
 
-static cudaError_t launch_one(int exp, const FusedArgs* reqs, const BatchTile* tiles, uint32_t nt, uint32_t* counter,
+static cudaError_t launch_one(int cls, const FusedArgs* reqs, const BatchTile* tiles, uint32_t nt, uint32_t* counter,
                               int grid, bool first, cudaStream_t st)
 {
-    switch (exp) {
+    switch (cls) {
     case 6: return launch_batch_t<6>(reqs, tiles, nt, counter, grid, first, st);
     case 7: return launch_batch_t<7>(reqs, tiles, nt, counter, grid, first, st);
     case 8: return launch_batch_t<8>(reqs, tiles, nt, counter, grid, first, st);
     case 9: return launch_batch_t<9>(reqs, tiles, nt, counter, grid, first, st);
-    default: return launch_batch_hi(exp, reqs, tiles, nt, counter, grid, first, st);
+    default: return launch_batch_hi(cls, reqs, tiles, nt, counter, grid, first, st);
     }
 }
 
@@ -43,7 +43,7 @@ cudaError_t launch_batch(const FusedArgs* d_reqs, const BatchTile* d_tiles, cons
         return launch_batch_all(d_reqs, d_tiles, tiles, d_counter, grid, st);
     for (int i = 0; i < k.count; ++i) {
         const BatchClasses::Class& c = k.cls[i];
-        const cudaError_t e = launch_one(c.exp, d_reqs, d_tiles + c.begin, c.tiles, d_counter + i,
+        const cudaError_t e = launch_one(c.id, d_reqs, d_tiles + c.begin, c.tiles, d_counter + i,
                                          (int)std::min<uint32_t>((uint32_t)grid, c.tiles), i == 0, st);
         if (e != cudaSuccess) return e;
     }

@@ -2,7 +2,8 @@
 //
 // A complex FFT of P points carries either two consecutive real frames of
 // N = P samples (z = y_a + i y_b, "pair") or one frame of N = 2P samples
-// (z[m] = y[2m] + i y[2m+1], "single").  P = r1 r2 16, 32 points per thread,
+// (z[m] = y[2m] + i y[2m+1], "single"; mirror_paired says which calls take
+// which).  P = r1 r2 16, 32 points per thread,
 // T = P / 32 threads per transform, in three stages with two exchanges through
 // shared memory.  With n = n0 + 16 n1 + 16 r2 n2 and k = k0 + r1 k1 + G k2
 // (G = r1 r2 = P / 16):
@@ -27,11 +28,13 @@
 // 15, 10 of 31, one rounding more each); the exchanges in place, which takes
 // three barriers per transform instead of five and no padding.
 // 1e8 samples, Hamming, before -> after (us; power at overlap 0.5, power at
-// 0.75, half-complex at 0.5): 2^12 312 -> 275, 601 -> 530, 206 -> 184; 2^13
-// 339 -> 298, 653 -> 567, 209 -> 199; 2^14 388 -> 319, 730 -> 621, 256 -> 203;
+// 0.75, half-complex at 0.5): 2^12 312 -> 275, 601 -> 530, 206 -> 185; 2^13
+// 339 -> 298, 653 -> 567, 209 -> 200; 2^14 388 -> 319, 730 -> 621, 256 -> 203;
 // 2^15 402 -> 361, 777 -> 699, 269 -> 239.  At 2^11 a frame is one warp of the
 // one-frame kernel, which has a single exchange and no barrier: 242 us against
-// 254 for this plan.
+// 254 for this plan.  Half-complex at 2^12 and 2^13 as a pair: 177 and 192 us, but
+// a quiet frame beside a loud one then loses digits (8e-4 of its norm at 1e-4 of
+// its neighbour's level, 1.4e-7 in the single form).
 //
 // Per frame it implements the reference's Overlap_Common -> Window_* ->
 // DCRemove_Common -> Stockham FFT -> toPower / toHalfComplexFormat
@@ -48,7 +51,10 @@ struct MirrorCfg {
 };
 __host__ __device__ constexpr MirrorCfg mirror_cfg(int lp)
 {
-    return lp == 12 ? MirrorCfg{12, 16, 16} : (lp == 13 ? MirrorCfg{13, 32, 16} : MirrorCfg{14, 32, 32});
+    return lp == 11   ? MirrorCfg{11, 16, 8}
+           : lp == 12 ? MirrorCfg{12, 16, 16}
+           : lp == 13 ? MirrorCfg{13, 32, 16}
+                      : MirrorCfg{14, 32, 32};
 }
 __host__ __device__ constexpr bool mirror_supported(int exp) { return exp >= 12 && exp <= 15; }
 __host__ __device__ constexpr int mirror_T(int lp) { return 1 << (lp - 5); }
@@ -74,9 +80,9 @@ __host__ __device__ constexpr int mirror_gpc(int lp) { return mirror_threads(lp)
 // Above it stays in global memory: its size would come out of the L1 that the
 // loads in flight need (2^13 298 -> 319 us; 2^15, half of it, 364 -> 404).
 __host__ __device__ constexpr bool mirror_smem_window(int exp) { return exp == 12; }
-__host__ __device__ constexpr size_t mirror_smem_bytes(int exp)
+__host__ __device__ constexpr size_t mirror_smem_bytes(int exp, bool pair)
 {
-    const int lp = mirror_lp(exp);
+    const int lp = mirror_lp(exp, pair);
     return ((size_t)mirror_gpc(lp) * 8 << lp) + (size_t)mirror_tab_size(lp) * 8 +
            (mirror_smem_window(exp) ? (size_t)4 << exp : 0) + (size_t)(mirror_threads(lp) / 32) * 8;
 }
@@ -113,11 +119,11 @@ __device__ __forceinline__ void mirror_twiddles(const float2* tab, int stride, F
     });
 }
 
-template <int EXP>
+template <int EXP, bool PAIR_>
 struct Mirror {
-    static constexpr bool PAIR = mirror_paired(EXP);
+    static constexpr bool PAIR = PAIR_;
     static constexpr int N = 1 << EXP, H = N / 2;
-    static constexpr int LP = mirror_lp(EXP), P = 1 << LP;
+    static constexpr int LP = mirror_lp(EXP, PAIR), P = 1 << LP;
     static constexpr int R1 = mirror_cfg(LP).r1, R2 = mirror_cfg(LP).r2;
     static constexpr int T = mirror_T(LP), G = P / 16;
 
@@ -214,9 +220,13 @@ struct Mirror {
     // Place of a point in the exchange buffer: n0 + 16 d1 + (P / r1) d2, d2
     // being n2 and then k0, d1 n1 and then k1, with the low four bits XORed by
     // a function of d2 so that the 16 points a half-warp touches lie in 16
-    // banks in every stage: (n0), (n0 mod 8, low bit of d2) or (n0), and (d2).
+    // banks in every stage: (n0), (n0 mod 8 or 4, low bits of d2) or (n0), and (d2).
     // (Stage 3's mirrored groups step d1 in one lane of 16: one conflict.)
-    static __host__ __device__ constexpr int swz(int d2) { return ((d2 >> 1) & 7) | ((d2 & 1) << 3); }
+    static __host__ __device__ constexpr int swz(int d2)
+    {
+        if (R2 == 8) return (d2 >> 2) | ((d2 & 2) << 1) | ((d2 & 1) << 3);  // d2 < 16
+        return ((d2 >> 1) & 7) | ((d2 & 1) << 3);
+    }
 
     // In: the windowed points (slot()).  Out: v[k2] = Z[t + G k2] and v[16 + j] =
     // Z[G - t + G ((j - 1) mod 16)] (thread 0: Z[G/2 + ..]).
@@ -250,6 +260,23 @@ struct Mirror {
             dft_inreg<32, 32, 0, 1>(v);
 #pragma unroll
             for (int k1 = 0; k1 < 32; ++k1) b[16 * k1] = v[k1];
+        } else if constexpr (R2 == 8) {
+            // groups (n0 + 4 i, k0), n0 < 4, i < 4, of one set of twiddles
+            const int k0 = t >> 2, m0 = swz(k0);
+            float2* const b = buf + S * k0 + ((t & 3) ^ (m0 & 3));
+            const int h = m0 & 12;  // place of n0 + 4 i in a run of 16: (4 i) ^ h from b
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[8 * i] = b[(4 * i) ^ h];
+            mirror_twiddles<8>(tw2 + k0, R1, [&](auto mc, float2 w) {
+                constexpr int m = decltype(mc)::value;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[8 * i + m] = cmul(b[((4 * i) ^ h) + 16 * m], w);
+            });
+            static_for<0, 4>([&](auto ic) { dft_inreg<32, 8, 8 * decltype(ic)::value, 1>(v); });
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int k1 = 0; k1 < 8; ++k1) b[((4 * i) ^ h) + 16 * k1] = v[8 * i + k1];
         } else {
             // groups (n0, k0) and (n0 + 8, k0), n0 < 8, of one set of twiddles
             const int k0 = t >> 3, m0 = swz(k0);
@@ -323,7 +350,7 @@ struct Mirror {
 template <int EXP, int OUTK>
 __device__ __forceinline__ void mirror_store_pair(const float2 (&v)[32], const FusedArgs& a, uint64_t fa, bool act_b, int t)
 {
-    using K = Mirror<EXP>;
+    using K = Mirror<EXP, true>;
     constexpr int N = K::N, H = K::H;
     float2* const o2 = reinterpret_cast<float2*>(a.out);
     const uint64_t fla = fa * (uint64_t)N, flb = fla + N;
@@ -385,7 +412,7 @@ __device__ __forceinline__ void mirror_store_pair(const float2 (&v)[32], const F
 template <int EXP, int OUTK>
 __device__ __forceinline__ void mirror_store_single(const float2 (&v)[32], const FusedArgs& a, uint64_t f, float2 wt, int t)
 {
-    using K = Mirror<EXP>;
+    using K = Mirror<EXP, false>;
     constexpr int N = K::N, M = K::H;
     float2* const o2 = reinterpret_cast<float2*>(a.out);
     const uint64_t fl = f * (uint64_t)N;
@@ -446,7 +473,7 @@ __device__ __forceinline__ void mirror_store_single(const float2 (&v)[32], const
 }
 
 // shared memory of a CTA, and group lp's parts of it
-template <int EXP>
+template <int EXP, bool PAIR>
 struct MirrorSmem {
     float2* buf;  // the group's exchange buffer
     float2* tab;  // twiddle tables
@@ -454,7 +481,7 @@ struct MirrorSmem {
     float2* red;  // the group's partial means
     __device__ __forceinline__ MirrorSmem(float2* smem, int lp)
     {
-        constexpr int LP = mirror_lp(EXP);
+        constexpr int LP = mirror_lp(EXP, PAIR);
         buf = smem + ((size_t)lp << LP);
         tab = smem + ((size_t)mirror_gpc(LP) << LP);
         win = reinterpret_cast<float*>(tab + mirror_tab_size(LP));
@@ -464,11 +491,11 @@ struct MirrorSmem {
 
 // Transform p of the request by the T threads of group lp: frames 2p and 2p + 1
 // (those below a.frames), or frame p in the single form.
-template <int EXP, int OUTK>
-__device__ __forceinline__ void mirror_transform(const FusedArgs& a, uint64_t p, const MirrorSmem<EXP>& sm,
+template <int EXP, bool PAIR, int OUTK>
+__device__ __forceinline__ void mirror_transform(const FusedArgs& a, uint64_t p, const MirrorSmem<EXP, PAIR>& sm,
                                                  const float* win, int lp, int t)
 {
-    using K = Mirror<EXP>;
+    using K = Mirror<EXP, PAIR>;
     constexpr int LP = K::LP;
     const float2* const tw2 = sm.tab;
     const float2* const tw3 = sm.tab + mirror_tw2_size(LP);
@@ -487,17 +514,23 @@ __device__ __forceinline__ void mirror_transform(const FusedArgs& a, uint64_t p,
     __syncwarp();  // thread 0 stored on a branch of its own; the barriers want whole warps
 }
 
+// threads of a CTA for an output kind
+__host__ __device__ constexpr int mirror_cta(int exp, int outk)
+{
+    return mirror_threads(mirror_lp(exp, mirror_paired(exp, outk)));
+}
+
 template <int EXP, int OUTK>
-__global__ void __launch_bounds__(mirror_threads(mirror_lp(EXP)), 512 / mirror_threads(mirror_lp(EXP)))
+__global__ void __launch_bounds__(mirror_cta(EXP, OUTK), 512 / mirror_cta(EXP, OUTK))
 stft_mirror_kernel(const FusedArgs a)
 {
-    using K = Mirror<EXP>;
+    using K = Mirror<EXP, mirror_paired(EXP, OUTK)>;
     constexpr int LP = K::LP, T = K::T, N = K::N, GPC = mirror_gpc(LP);
     constexpr int NT = mirror_threads(LP);
     extern __shared__ float4 smem4[];
     const int tid = threadIdx.x;
     const int lp = tid / T, t = tid - lp * T;
-    const MirrorSmem<EXP> sm(reinterpret_cast<float2*>(smem4), lp);
+    const MirrorSmem<EXP, K::PAIR> sm(reinterpret_cast<float2*>(smem4), lp);
     pdl_trigger();
     for (int i = tid; i < mirror_tab_size(LP); i += NT) sm.tab[i] = a.tw[i];
     const float* win = a.win;
@@ -517,7 +550,7 @@ stft_mirror_kernel(const FusedArgs a)
             const uint64_t s0 = FPT * (p + stride) * a.hop, end = s0 + (FPT - 1) * a.hop + N;
             prefetch_l2_span(a.x, s0, end < a.n ? end : a.n);
         }
-        mirror_transform<EXP, OUTK>(a, p, sm, win, lp, t);
+        mirror_transform<EXP, K::PAIR, OUTK>(a, p, sm, win, lp, t);
     }
 }
 
@@ -527,10 +560,10 @@ namespace ocs {
 template <int EXP, int OUTK>
 cudaError_t launch_mirror_t(const FusedArgs& a, int grid, cudaStream_t st)
 {
-    constexpr size_t sm = mirror_smem_bytes(EXP);
+    constexpr size_t sm = mirror_smem_bytes(EXP, mirror_paired(EXP, OUTK));
     const cudaError_t e = ensure_smem_attr<stft_mirror_kernel<EXP, OUTK>>(sm);
     if (e != cudaSuccess) return e;
-    return launch_pdl(stft_mirror_kernel<EXP, OUTK>, grid, mirror_threads(mirror_lp(EXP)), sm, st, a);
+    return launch_pdl(stft_mirror_kernel<EXP, OUTK>, grid, mirror_cta(EXP, OUTK), sm, st, a);
 }
 
 template <int EXP>
@@ -548,10 +581,10 @@ template <int EXP, int OUTK>
 int occupancy_mirror_t()
 {
     int blocks = 0;
-    constexpr size_t sm = mirror_smem_bytes(EXP);
+    constexpr size_t sm = mirror_smem_bytes(EXP, mirror_paired(EXP, OUTK));
     auto k = stft_mirror_kernel<EXP, OUTK>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, mirror_threads(mirror_lp(EXP)), sm) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, mirror_cta(EXP, OUTK), sm) != cudaSuccess)
         return 0;
     return blocks;
 }

@@ -5,7 +5,10 @@
 namespace ocs {
 
 bool pairx2_has(int exp, int outk) { return mirror_supported(exp) && outk != OUT_PLANES; }
-int pairx2_per_cta(int exp) { return mirror_gpc(mirror_lp(exp)); }
+static_assert(mirror_gpc(mirror_lp(12, false)) == 2 * mirror_gpc(mirror_lp(12, true)) &&
+                  mirror_gpc(mirror_lp(13, false)) == 2 * mirror_gpc(mirror_lp(13, true)),
+              "a CTA holds as many frames in either form");
+int pairx2_per_cta(int exp) { return mirror_gpc(mirror_lp(exp, exp <= 13)); }
 
 cudaError_t launch_pairx2(int exp, int outk, const FusedArgs& a, int grid, cudaStream_t st)
 {

@@ -8,8 +8,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 POWER, SERIAL, HALF = "", "--serial_power", "--half_complex_return"
 DENSE = " --layout=dense"
-ONE_REQUEST = [(e, POWER) for e in (6, 7, 8, 11, 14, 15)] + [(8, SERIAL)]
-BATCH = [(e, POWER) for e in (6, 7, 8, 11)] + [(8, SERIAL)]
+ONE_REQUEST = [(e, POWER) for e in (6, 7, 8, 11, 14, 15)] + [(8, SERIAL)] + [(e, HALF) for e in (6, 7, 8, 9, 11, 12, 13, 14, 15)]
+BATCH = ([(e, POWER) for e in (6, 7, 8, 11, 13)] + [(e, SERIAL) for e in range(6, 14)] +
+         [(e, HALF) for e in range(6, 14)])
 
 
 def _frames(exp, frames):
