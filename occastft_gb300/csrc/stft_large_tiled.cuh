@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(256, 2) large_tiled_columns_kernel(const Large
     const uint32_t tiles = M2 / TC;
     const uint64_t fg = blockIdx.x / tiles;
     const uint32_t c0 = (blockIdx.x % tiles) * TC;
+    pdl_trigger();
+    pdl_wait();
     for (int i = tid; i < C::ROWS * RA; i += 256) s_tw[i] = lt_w(a.tw1, M1, mirror_row_m(i / RA) * (i % RA));
     // stage 1: column c0 + sc, rows q + RB p
     const int sc = tid % TC, q = tid / TC;
@@ -224,6 +226,8 @@ large_tiled_rows_kernel(const LargeArgs a)
     const uint64_t fl = blockIdx.x / blocks;
     const uint32_t b = blockIdx.x % blocks;
     const uint64_t f = a.f0 + fl;
+    pdl_trigger();
+    pdl_wait();
     for (int i = tid; i < R::ROWS * 16; i += R::THREADS) s_tw[i] = lt_w(a.tw2, M2, mirror_row_m(i / 16) * (i % 16));
     const int r = tid & 15, t = tid >> 4;
     const uint32_t k1 = kLtTile * b + r;
