@@ -4,13 +4,13 @@
 namespace ocs {
 namespace {
 
-// Requests of a few frames, whose two grids find an SM for each CTA (152), overlap
-// each pass's launch with the pass before (launch_pdl): one frame, power /
-// half-complex, 2^16 12.4 / 14.4 -> 9.1 / 10.8 us, 2^18 18.1 / 20.2 -> 12.5 / 14.4
-// (the untiled passes: 18.9 / 18.8).  Beyond that, CTAs that wait share SMs with
-// CTAs that work while others are free (2^16, 17 frames 19.0 -> 21.9 us), and long
-// requests lose the room (2^18, 1e8 samples, 532 -> 540 us).
-constexpr uint64_t kOverlapCtas = 152;
+// Requests of a few frames, whose two grids and the next request's find an SM for
+// each CTA (half of 152 for one request), overlap each pass's launch with the pass
+// before (launch_pdl): one frame, power / half-complex, 2^16 12.4 / 14.4 -> 9.1 /
+// 10.8 us, 2^18 18.1 / 20.2 -> 12.5 / 14.4 (the untiled passes: 18.9 / 18.8).
+// Beyond that CTAs share SMs while others are free (2^17, 7 frames and 88 CTAs 18.8
+// -> 19.8 us), and long requests lose the room (2^18, 1e8 samples, 532 -> 540 us).
+constexpr uint64_t kOverlapCtas = 76;
 template <typename... P>
 cudaError_t launch_pass(bool overlap, void (*kernel)(P...), uint64_t grid, int threads, size_t smem, cudaStream_t st,
                         const LargeArgs& a)
