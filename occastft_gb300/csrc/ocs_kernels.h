@@ -136,6 +136,18 @@ constexpr int batch_class(int exp, int outk)
     return exp == 12 && !batch_mirror_paired(exp, outk) ? kBatchSingle12 : exp;
 }
 constexpr int batch_class_exp(int cls) { return cls & 31; }
+// The fewest frames of a tile: what a CTA of the body takes at a time, 16384
+// points in the lanes-per-frame, paired and mirror-group bodies, and of the
+// one-frame bodies, which take fewer, two rounds where one is 4096 points.  With
+// tiles of one round of the one-frame kernel six of eight warps idled at 2^7 and
+// half of the pairs at 2^9 and 2^10 (power, 8 requests: 2^9 21.4 -> 17.0 us, 2^10
+// 22.2 -> 18.1; half-complex at 2^7, 64 requests: 62 -> 56).
+constexpr uint64_t batch_min_frames(int exp, int outk)
+{
+    const bool wide = exp >= 12 || (outk == OUT_POWER && exp >= 7 && exp <= 10) ||
+                      (outk == OUT_POWER_SERIAL && (exp == 7 || exp == 8));
+    return (wide ? 16384u : 8192u) >> exp;
+}
 // the tiles of each class, in the order of the tile list; class i's queue
 // counter is d_counter[i]
 struct BatchClasses {

@@ -7,11 +7,26 @@ namespace ocs {
 
 size_t batch_smem_bytes() { return batch_smem(0); }
 bool batch_supports(int exp) { return exp >= kBatchMinExp && exp <= kBatchMaxExp; }
-// a tile is `groups` CTA-groups of frames (the host's autotuner picks the
-// count per batch mix; any count keeps tiles whole groups of every body)
-// -- at 2^13, where a CTA of the one-frame kernel holds one frame, groups of two,
-// as the mirror-group body holds
+// `groups` groups of frames, a group being what a CTA of the one-frame kernel
+// holds (two frames at 2^13, as the mirror-group body).  The host's autotuner
+// picks the count per batch mix, a power of two, and makes a tile no shorter than
+// batch_min_frames, so that tiles are whole rounds of every body and start on
+// whole pairs of frames.
 int batch_tile_frames(int exp, int groups) { return (exp == 13 ? 2 : fused_fpc(exp)) * groups; }
+
+static_assert(batch_min_frames(7, OUT_POWER) == 8 * TplCfg<7>::F && batch_min_frames(8, OUT_POWER) == 8 * TplCfg<8>::F,
+              "a round of the lanes-per-frame bodies");
+static_assert(batch_min_frames(9, OUT_POWER) == 2 * pair_ppc(9) && batch_min_frames(10, OUT_POWER) == 2 * pair_ppc(10),
+              "a round of the paired bodies");
+static_assert(batch_min_frames(12, OUT_POWER) == 2 * mirror_gpc(mirror_lp(12, true)) &&
+                  batch_min_frames(12, OUT_HALF) == mirror_gpc(mirror_lp(12, false)) &&
+                  batch_min_frames(13, OUT_HALF) == mirror_gpc(mirror_lp(13, false)),
+              "a round of the mirror-group bodies");
+static_assert(batch_min_frames(6, OUT_HALF) % fused_fpc(6) == 0 && batch_min_frames(7, OUT_HALF) % fused_fpc(7) == 0 &&
+                  batch_min_frames(8, OUT_HALF) % fused_fpc(8) == 0 && batch_min_frames(9, OUT_HALF) % fused_fpc(9) == 0 &&
+                  batch_min_frames(10, OUT_HALF) % fused_fpc(10) == 0 &&
+                  fused_fpc(11) % batch_min_frames(11, OUT_POWER) == 0,
+              "whole rounds of the one-frame bodies");
 
 int batch_occupancy()
 {

@@ -87,6 +87,9 @@ void classes(cudaStream_t st)
             last = exp;
             for (const auto& t : c.tiles) {
                 check(ocs::batch_class(t.exp, t.outk) == c.id, "tile's class");
+                // whole rounds of the tile's body, but for a request's last tile
+                const uint64_t least = ocs::batch_min_frames(t.exp, t.outk);
+                check(t.f0 % least == 0 && (t.nframes % least == 0 || t.f0 + t.nframes == t.frames), "tile's frames");
                 if (exp >= 12)
                     check(t.plan == ocs::mirror_plan_id(exp, ocs::batch_mirror_paired(exp, t.outk)), "table");
                 else if (exp != 7 && exp != 11)
