@@ -14,6 +14,7 @@
 #include <cstring>
 #include <random>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -143,6 +144,38 @@ void failed_launch(cudaStream_t st)
     cudaStreamDestroy(other);
 }
 
+// Two batches of the same windows and size whose frames lie in different
+// windows: the tile length kept for the first must not stretch the second's.
+void tune_key(cudaStream_t st)
+{
+    setenv("OCS_AUTOTUNE", "1", 1);
+    fake::tile_us = 40;  // fewer, longer tiles are faster: the tuner takes the longest
+    const uint64_t many = 2100, few = 20;
+    auto longest = [&](uint64_t at8, uint64_t at12) {
+        Batch b;
+        b.add(at8 * 128, 8, 0.5f, "");
+        b.add(at12 * 2048, 12, 0.5f, "");
+        b.seal();
+        check(b.run(st) == OCS_OK, "launch");
+        cudaStreamSynchronize(st);
+        check(b.right(), "outputs");
+        // the classes of the last launch
+        std::vector<fake::ClassLaunch> l = fake::take_class_launches();
+        uint64_t most8 = 0, most12 = 0;
+        for (size_t i = l.size() - 2; i < l.size(); ++i)
+            for (const auto& t : l[i].tiles) {
+                uint64_t& m = t.exp == 8 ? most8 : most12;
+                m = std::max(m, t.nframes);
+            }
+        return std::make_pair(most8, most12);
+    };
+    // mostly at 2^12, 8 groups make enough tiles: up to 64 groups
+    check(longest(few, many).second == (uint64_t)ocs::batch_tile_frames(12, 64), "the first batch's longest tile");
+    // mostly at 2^8, they do not: no tile above 8 groups
+    check(longest(many, few).first <= (uint64_t)ocs::batch_tile_frames(8, 8), "the second batch's tiles");
+    fake::tile_us = 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -155,6 +188,7 @@ int main(int argc, char** argv)
     if (what == "classes") classes(st);
     else if (what == "one_request") one_request(st);
     else if (what == "failed_launch") failed_launch(st);
+    else if (what == "tune_key") tune_key(st);
     else check(false, "unknown check");
     cudaStreamSynchronize(st);
     cudaStreamDestroy(st);

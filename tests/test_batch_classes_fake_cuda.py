@@ -13,7 +13,7 @@ CSRC = os.path.join(ROOT, "occastft_gb300", "csrc")
 SOURCES = [os.path.join(CSRC, "ocs_api.cpp"), os.path.join(CSRC, "ocs_host.cpp"),
            os.path.join(FAKE, "fake_runtime.cpp"), os.path.join(FAKE, "batch_class_kernels.cpp"),
            os.path.join(FAKE, "batch_class_checks.cpp")]
-CHECKS = ["classes", "one_request", "failed_launch"]
+CHECKS = ["classes", "one_request", "failed_launch", "tune_key"]
 
 
 @pytest.fixture(scope="module")
