@@ -236,7 +236,7 @@ namespace internal {
 // Forgets the per-device set-up (called by ocs_shutdown): after a
 // cudaDeviceReset the module is loaded again, possibly at another address,
 // and its tables are gone, so the next call sets the device up afresh.  The
-// large windows' pool and side streams go with it.
+// large windows' scratch pool goes with it.
 void noalloc_forget_devices()
 {
     large_release();

@@ -1,5 +1,7 @@
 // STFT for windows 2^16 .. 2^30 (sm_103a): a four-step FFT in two launches
-// up to 2^22, three above.
+// up to 2^22, three above.  Windows 2^16 .. 2^19 run the tiled passes of
+// stft_large_tiled.cuh; the ones here take 2^20 and up.  The scratch of all of
+// them, and the chunks a request is cut into, are at the end of this file.
 //
 // One frame of N real samples is the M = N/2 point complex FFT of
 // z[m] = y[2m] + i y[2m+1] plus the real-input untangle, as in the fused
@@ -11,7 +13,7 @@
 // X[k + M] = (Z[k] + conj Z[M-k]) - W_N^k (...) (the window table carries the
 // untangle's factor 1/2).
 //
-// Column pass: a CTA owns 16 (windows 2^16, 2^17) or 8 consecutive columns
+// Column pass: a CTA owns 16 (columns of 256 points) or 8 consecutive columns
 // of one frame.  It reads the frame's samples row by row (128 or 64
 // contiguous bytes per row), applies the
 // window, runs 8 M1-point FFTs with the fused kernels' Stockham core, applies
@@ -59,9 +61,8 @@ __host__ __device__ constexpr int large_col_stride(int exp1)
 }
 // Row-pass buffers: row r starts at r * large_row_stride + large_row_shift(r),
 // the stride a multiple of 16 float2 and the shift 0, 8, 4, 12, 2, 10, 6, 14
-// for r mod 8.  The four rows a warp transforms at window 2^8 (8 lanes per row
-// on 8 consecutive slots) then tile the 16 bank pairs twice, and so do the
-// output loop's reads of 8 rows at 4 consecutive columns.
+// for r mod 8, so that the output loop's reads of 8 rows at 4 consecutive
+// columns tile the 16 bank pairs twice.
 __host__ __device__ constexpr int large_row_stride(int exp2) { return (fused_buf_stride(exp2) + 14 + 15) / 16 * 16; }
 __device__ __forceinline__ int large_row_shift(int r) { return 8 * (r & 1) + 4 * ((r >> 1) & 1) + 2 * ((r >> 2) & 1); }
 
@@ -75,13 +76,13 @@ __device__ __forceinline__ float2 tw2l(const float2* lo, const float2* hi, uint6
 }
 
 // ---------------------------------------------------------------- column pass
-// Column FFTs of up to 512 points (windows 2^16 .. 2^19) keep the CTA's
+// Column FFTs of up to 512 points (windows 2^23 .. 2^29) keep the CTA's
 // window coefficients in registers and take 4 consecutive frames of the same
 // columns per CTA; the larger ones (more chunks per thread, or 1024 threads
 // at 64 registers) take one frame per CTA and read the window each time.
 //
 // A CTA owns 16 columns (rows of 128 bytes, 8 lanes per row) where that keeps
-// it at 256 threads (column FFTs of 256 points, windows 2^16 and 2^17), else
+// it at 256 threads (column FFTs of 256 points, windows 2^23 .. 2^27), else
 // 8: each warp-wide row load then touches half as many cache lines.
 __host__ __device__ constexpr int large_col_tile(int exp1)
 {
@@ -512,8 +513,6 @@ cudaError_t launch_columns(int l1, const LargeArgs& a, uint64_t frames, cudaStre
 cudaError_t launch_rows(int l3, int outk, const LargeArgs& a, uint64_t frames, cudaStream_t st)
 {
     switch (l3 + 1) {
-    case 8: return launch_rows_e<8>(outk, a, frames, st);
-    case 9: return launch_rows_e<9>(outk, a, frames, st);
     case 10: return launch_rows_e<10>(outk, a, frames, st);
     case 11: return launch_rows_e<11>(outk, a, frames, st);
     default: return cudaErrorInvalidValue;
@@ -528,8 +527,6 @@ cudaError_t launch_middle(int l2, const LargeArgs& a, uint64_t frames, cudaStrea
     case 8: return launch_middle_t<8>(a, frames, st);
     case 9: return launch_middle_t<9>(a, frames, st);
     case 10: return launch_middle_t<10>(a, frames, st);
-    case 11: return launch_middle_t<11>(a, frames, st);
-    case 12: return launch_middle_t<12>(a, frames, st);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -537,31 +534,42 @@ cudaError_t launch_middle(int l2, const LargeArgs& a, uint64_t frames, cudaStrea
 }  // namespace
 
 // windows of the tiled kernels (stft_large_tiled.cuh)
-static bool large_tiled(int exp) { return exp >= 16 && exp <= 19; }
+static constexpr bool large_tiled(int exp) { return exp >= 16 && exp <= 19; }
 cudaError_t launch_large_tiled(int l1, int l2, int outk, const LargeArgs& a, uint64_t frames, cudaStream_t st);
 
 bool large_supports(int exp) { return exp >= kLargeMinExp && exp <= kLargeMaxExp; }
 
 // Two passes up to 2^22 (column FFT 2^(exp/2), rows of the rest).  Above,
-// rows of Q = 2^l3 points (l3 <= 10, the largest row pass), a column FFT of
-// 2^l1 (8 <= l1 <= 11) and a middle FFT of 2^l2 (5 <= l2 <= 11), l1 >= l2 as
-// close as the ranges allow.
-LargePlan large_plan(int exp)
+// rows of Q = 2^l3 points (the largest row pass, 2^10, but at 2^23), a column FFT
+// of 2^l1 and a middle FFT of 2^l2, l1 >= l2 as close as l1 >= 8 allows.
+static constexpr LargePlan plan_of(int exp)
 {
     if (large_tiled(exp)) {
         const int l2 = exp == 16 ? 7 : 8;
         return LargePlan{2, exp - 1 - l2, 0, l2};
     }
     if (exp <= 22) return LargePlan{2, large_l1(exp), 0, large_l2(exp)};
-    const int total = exp - 1;
-    for (int l3 = 10; l3 >= 7; --l3) {
-        const int rest = total - l3;
-        const int l1 = (rest + 1) / 2 < 8 ? 8 : ((rest + 1) / 2 > 11 ? 11 : (rest + 1) / 2);
-        const int l2 = rest - l1;
-        if (l2 >= 5 && l2 <= 11) return LargePlan{3, l1, l2, l3};
+    for (int l3 = 10; l3 >= 9; --l3) {
+        const int rest = exp - 1 - l3;
+        const int l1 = (rest + 1) / 2 < 8 ? 8 : (rest + 1) / 2;
+        if (rest - l1 >= 5) return LargePlan{3, l1, rest - l1, l3};
     }
     return LargePlan{0, 0, 0, 0};
 }
+// every window's passes are among the ones launch_columns, launch_middle and
+// launch_rows hold
+static constexpr bool plans_held()
+{
+    for (int exp = 20; exp <= kLargeMaxExp; ++exp) {
+        const LargePlan p = plan_of(exp);
+        if (p.passes == 0 || p.l1 < 8 || p.l1 > 11 || p.l3 < 9 || p.l3 > 10) return false;
+        if (p.passes == 3 && (p.l2 < 5 || p.l2 > 9)) return false;
+        if (p.l1 + p.l2 + p.l3 != exp - 1) return false;
+    }
+    return true;
+}
+static_assert(plans_held(), "");
+LargePlan large_plan(int exp) { return plan_of(exp); }
 
 cudaError_t build_two_level(float2* lo, float2* hi, uint64_t L, cudaStream_t st)
 {
