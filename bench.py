@@ -14,8 +14,8 @@ metric is input samples per second (Gsamples/s).
            result are inside the timed region.
   roofline algorithmic bytes (4 n + 4 qt N) per launch / mean launch time,
            against the measured HBM copy bandwidth.
-  sweep    the rest of the config: windows 2^6..2^15 x {Hamming, Blackman} x
-           {power, half-complex}, device-resident.
+  sweep    the rest of the config: windows 2^6..2^22 x {Hamming, Blackman} x
+           {power, half-complex}, device-resident; with the other legs on stderr.
 
 `--impl reference` times the reference's own CPU implementation of the path
 (its OpenMP runner built from source when available, else the pinned oracle

@@ -89,7 +89,16 @@ int ocs_activate(const float* in, uint64_t n, int window_size_exp, float overlap
  * kernel launch on `stream`, asynchronous.  With --precision=tc-fp16 a wait
  * inside the tensor-core kernel that gives up (after about a second) is
  * reported as OCS_ETIMEDOUT by ocs_activate at once and, since this call
- * does not synchronise, by the next tensor-core call of this function. */
+ * does not synchronise, by the next tensor-core call of this function.
+ * Windows from 2^16 up take stream-ordered scratch from a memory pool of the
+ * library's own, not from the device's current pool.  The pool keeps up to
+ * 1 GB of idle memory until ocs_shutdown; OCS_LARGE_SCRATCH_MB bounds what a
+ * request takes.  A captured request's scratch belongs to its graph.
+ * Power at 2^9, 2^10, 2^12 and 2^13 carries two neighbouring frames in one
+ * FFT, as may half-complex at 2^10: a frame much quieter than its neighbour
+ * is rounded relative to the louder one, and infinities and NaN reach both.
+ * OCS_KERNEL=single in the environment keeps these calls to one frame per
+ * FFT. */
 int ocs_activate_device(const float* d_in, uint64_t n, int window_size_exp, float overlap_ratio,
                         const char* options, float* d_out, uint64_t out_cap, void* stream);
 
@@ -101,7 +110,8 @@ int ocs_activate_device(const float* d_in, uint64_t n, int window_size_exp, floa
  * fastest, as the first call of that shape would.  *variant (may be NULL)
  * receives the variant the whole request runs: 0 one frame per FFT, 1 the
  * same with staged I/O, 2 two frames per FFT, 3 lanes per frame, 4 the
- * mirror-group kernel; -1 where the shape has one form (windows
+ * mirror-group kernel (two frames per transform for power at 2^12 and 2^13,
+ * one otherwise); -1 where the shape has one form (windows
  * above 2^15, tensor-core precisions).  With OCS_AUTOTUNE=0 nothing is timed
  * and the default variant is reported.  Synchronous. */
 int ocs_plan_tune(uint64_t n, int window_size_exp, float overlap_ratio, const char* options, int* variant);
@@ -149,19 +159,19 @@ typedef struct ocs_request {
 int ocs_batch_prepare(const ocs_request* reqs, int count);
 
 /* Runs all valid requests (windows 2^6..2^13) as tiles of persistent
- * launches on `stream`, one per window size or one for all of them where the
- * batch is small (requests with larger windows get their own
- * fused launch on the same stream).  Asynchronous.  Returns OCS_OK when the
- * launch was issued; per-request problems land in reqs[i].status.
+ * launches on `stream`, one per window size (two at 2^12 with mixed outputs)
+ * or one for all of them where the batch is small (requests with larger
+ * windows get their own fused launch on the same stream).  Power at 2^9, 2^10
+ * and 2^12 carries two frames in one FFT here.  Asynchronous.  Returns OCS_OK
+ * when the launches were issued; per-request problems land in reqs[i].status.
  * Under stream capture it uses the buffers the last ocs_batch_prepare set
  * aside (OCS_ENOMEM if there are none, or they are too small) and keeps them
  * until ocs_shutdown, so the graph replays its own requests whatever batches
  * run after the capture.  Replays of one graph must not overlap each other on
  * the GPU (they share those buffers); replays and other batches may.
  * The first call outside capture for a new mix of window sizes and batch
- * size times four tile lengths on these
- * requests, running the batch about a dozen times, and waits for that; the
- * outputs are the same for every length.  OCS_AUTOTUNE=0 skips this. */
+ * size times four tile lengths on these requests, running the batch about a
+ * dozen times, and waits for that; the outputs are the same for every length.  OCS_AUTOTUNE=0 skips this. */
 int ocs_batch_device(ocs_request* reqs, int count, void* stream);
 
 /* Same as ocs_batch_device, for callers that must not allocate GPU memory

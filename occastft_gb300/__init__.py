@@ -272,7 +272,7 @@ def batch_prepare(reqs) -> None:
 
 
 def batch_device(reqs, stream=None) -> list:
-    """Persistent launches over all requests, one per window size at most; returns the per-request status codes."""
+    """Persistent launches over all requests, one per window size (two at 2^12) at most; returns the per-request status codes."""
     _check(lib().ocs_batch_device(ctypes.cast(reqs, ctypes.c_void_p), len(reqs), _stream_handle(stream)))
     return [r.status for r in reqs]
 

@@ -21,7 +21,7 @@
 // group G/2.
 //
 // What bounds it: latency at 16 warps per SM, with the L1/shared-memory pipe at
-// 47% and issue at 47% (ncu, 2^12).  A transform's 32 points per thread take
+// 51% and issue at 51% (ncu, 2^12, overlap 0.75).  A transform's 32 points per thread take
 // half the registers of an SM, so the plan saves wavefronts, instructions and
 // barriers per sample: no third exchange (a third of the exchange traffic);
 // the twiddles of a stage from a few table entries and products (6 loads of
