@@ -45,7 +45,7 @@ def test_tuner_keeps_the_accuracy(ocs_lib, exp, opts):
     """The tuner's own pick never puts two frames in one FFT where that is not
     the window's rule, nor the two-level twiddles beside a one-frame mirror."""
     half = HALF in opts
-    pair_ok = exp == 10 if half else exp in (9, 10, 12, 13)
+    pair_ok = exp in (6, 10) if half else exp in (6, 9, 10, 12, 13)
     for n in (1 << 17, 1 << 21, 1 << 24):
         v = ocs_lib.plan_tune(n, exp, 0.5, opts)
         two = v == PAIR or (v == MIRROR and exp <= 13 and not half)
