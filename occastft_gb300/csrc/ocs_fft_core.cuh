@@ -117,6 +117,16 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
+// A translation unit that defines OCS_SCALAR_COMPLEX gets the scalar forms (its
+// device code is its own; nothing is linked across units).
+#ifdef OCS_SCALAR_COMPLEX
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 cmul(float2 a, float2 b)
+{
+    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+#else
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return add2(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return add2(a, make_float2(-b.x, -b.y)); }
 // a b; the product with b.y is the one that rounds, so that multiplying by a
@@ -125,6 +135,7 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
     return fma2(a, bc2(b.x), mul2(make_float2(-a.y, a.x), bc2(b.y)));
 }
+#endif
 // a + conj b and (a - conj b) / i: the two halves of the separations below
 __device__ __forceinline__ float2 cadd_conj(float2 a, float2 b) { return add2(a, make_float2(b.x, -b.y)); }
 __device__ __forceinline__ float2 cdif_conj(float2 a, float2 b)
@@ -145,6 +156,18 @@ __device__ __forceinline__ float2 twc(float2 a)
         return make_float2(a.y, -a.x);
     } else if constexpr (4 * j == 3 * L) {  // +i
         return make_float2(-a.y, a.x);
+#ifdef OCS_SCALAR_COMPLEX
+    } else if constexpr (8 * j == L) {  // (1-i)/sqrt2
+        return make_float2((a.x + a.y) * kRsqrt2, (a.y - a.x) * kRsqrt2);
+    } else if constexpr (8 * j == 3 * L) {  // (-1-i)/sqrt2
+        return make_float2((a.y - a.x) * kRsqrt2, -(a.x + a.y) * kRsqrt2);
+    } else {
+        constexpr float c = (float)cx_cos(kTwoPi * j / L);
+        constexpr float s = (float)cx_sin(kTwoPi * j / L);
+        // (x + iy)(c - is)
+        return make_float2(a.x * c + a.y * s, a.y * c - a.x * s);
+    }
+#else
     } else if constexpr (8 * j == L) {  // (1-i)/sqrt2
         return mul2(add2(a, make_float2(a.y, -a.x)), bc2(kRsqrt2));
     } else if constexpr (8 * j == 3 * L) {  // (-1-i)/sqrt2
@@ -156,6 +179,7 @@ __device__ __forceinline__ float2 twc(float2 a)
         if constexpr (c * c >= s * s) return fma2(a, bc2(c), mul2(make_float2(a.y, -a.x), bc2(s)));
         else return fma2(make_float2(a.y, -a.x), bc2(s), mul2(a, bc2(c)));
     }
+#endif
 }
 
 constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
