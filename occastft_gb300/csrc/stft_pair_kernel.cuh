@@ -210,9 +210,10 @@ stft_pair_kernel(const FusedArgs a)
 
     const uint64_t pairs = (a.frames + 1) / 2;
     for (uint64_t pbase = (uint64_t)blockIdx.x * PPC; pbase < pairs; pbase += (uint64_t)gridDim.x * PPC) {
-        // L2 prefetch of the pair this group takes next: samples of frames 2q and 2q + 1
+        // L2 prefetch of the pair this group takes next: samples of frames 2q and
+        // 2q + 1, where frames overlap (see the one-frame kernel)
         const uint64_t q = pbase + (uint64_t)gridDim.x * PPC + lp;
-        if (t == 0 && q < pairs) {
+        if (t == 0 && q < pairs && a.hop < (uint64_t)(1 << EXP)) {
             const uint64_t s0 = 2 * q * a.hop;
             const uint64_t end = s0 + a.hop + (uint64_t)(1 << EXP);
             prefetch_l2_span(a.x, s0, end < a.n ? end : a.n);
