@@ -95,9 +95,9 @@ int ocs_activate(const float* in, uint64_t n, int window_size_exp, float overlap
  * 1 GB of idle memory until ocs_shutdown; OCS_LARGE_SCRATCH_MB bounds what a
  * request takes.  A captured request's scratch belongs to its graph.
  * Power at 2^9, 2^10, 2^12 and 2^13 carries two neighbouring frames in one
- * FFT, as may half-complex at 2^10 and short requests at 2^6: a frame much
- * quieter than its neighbour is rounded relative to the louder one, and
- * infinities and NaN reach both.  OCS_KERNEL=single in the environment keeps
+ * FFT, as may half-complex at 2^10 (long dense requests at 2^8 and 2^9 too)
+ * and short requests at 2^6: a frame much quieter than its neighbour is
+ * rounded relative to the louder one, and infinities and NaN reach both.  OCS_KERNEL=single in the environment keeps
  * these calls to one frame per FFT. */
 int ocs_activate_device(const float* d_in, uint64_t n, int window_size_exp, float overlap_ratio,
                         const char* options, float* d_out, uint64_t out_cap, void* stream);
