@@ -595,12 +595,12 @@ __device__ __forceinline__ void fused_group_frames(const FusedArgs& a, uint64_t 
     }
 }
 
-// L2 prefetch of frame f (the frame this thread's group takes next), issued
-// by the group's first thread
+// L2 prefetch of frame f (the frame this thread's group takes next) below
+// `frames`, issued by the group's first thread
 template <int EXP>
-__device__ __forceinline__ void fused_prefetch_next(const FusedArgs& a, uint64_t f, int t)
+__device__ __forceinline__ void fused_prefetch_next(const FusedArgs& a, uint64_t f, int t, uint64_t frames)
 {
-    if (t == 0 && f < a.frames) {
+    if (t == 0 && f < frames) {
         const uint64_t s0 = f * a.hop;
         const uint64_t s1 = s0 + (uint64_t)(1 << EXP) < a.n ? s0 + (uint64_t)(1 << EXP) : a.n;
         prefetch_l2_span(a.x, s0, s1);
@@ -640,11 +640,11 @@ stft_fused_kernel(const FusedArgs a)
         // Frames that do not overlap are read once and gain nothing from the L2
         // prefetch, which then only competes with the loads and stores: power,
         // 1e8 samples, with it -> without, overlap 0 / -0.5: 2^9 (paired) 147 / 115
-        // -> 134 / 93 us, 2^10 (paired) 152 / 114 -> 128 / 89, 2^11 151 / 104 -> 129 /
-        // 88; at overlap 0.25 and 0.5 it gives 1 to 10%.
+        // -> 134 / 93 us, 2^11 151 / 104 -> 129 / 88; at overlap 0.25 and 0.5 it gives
+        // 1 to 10%.
+        const uint64_t ahead = a.hop < (uint64_t)(1 << EXP) ? a.frames : 0;  // frames to prefetch
         for (uint64_t fbase = (uint64_t)blockIdx.x * FPC; fbase < a.frames; fbase += (uint64_t)gridDim.x * FPC) {
-            if (a.hop < (uint64_t)(1 << EXP))
-                fused_prefetch_next<EXP>(a, fbase + (uint64_t)gridDim.x * FPC + lf, t);
+            fused_prefetch_next<EXP>(a, fbase + (uint64_t)gridDim.x * FPC + lf, t, ahead);
             fused_group_frames<EXP, OUTK>(a, fbase, buf, red, tw, win2, tid, lf, t);
         }
     } else {
@@ -653,7 +653,7 @@ stft_fused_kernel(const FusedArgs a)
         pdl_wait();
         const float2* win2 = reinterpret_cast<const float2*>(a.win);
         for (uint64_t fbase = (uint64_t)blockIdx.x * FPC; fbase < a.frames; fbase += (uint64_t)gridDim.x * FPC) {
-            fused_prefetch_next<EXP>(a, fbase + (uint64_t)gridDim.x * FPC + lf, t);
+            fused_prefetch_next<EXP>(a, fbase + (uint64_t)gridDim.x * FPC + lf, t, a.frames);
             fused_group_frames<EXP, OUTK>(a, fbase, buf, red, tw, win2, tid, lf, t);
         }
     }
